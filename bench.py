@@ -478,7 +478,7 @@ def main():
                     help="run only the serving leg (--serve-requests over --serve-systems) and print it")
     ap.add_argument("--no-extras", action="store_true", help="skip e2e/plain/cpu/serving legs")
     ap.add_argument("--no-autotune", action="store_true",
-                    help="accepted and without effect: launch shapes follow from the system")
+                    help="FP32 descreening sums over 128 columns whatever the size of the run")
     args = ap.parse_args()
     if args.impl == "reference":
         run_reference(args)

@@ -285,8 +285,9 @@ typedef struct rstg_system_opts {
   int64_t max_batch_frames; /* frames per device batch (0: as many as fit a
                               2 GB share of device memory, at most 256)      */
   int32_t use_graphs;      /* capture each batch's launch sequence (default 1) */
-  int32_t autotune;        /* no effect: every launch shape follows from the
-                              sizes (kept so that the struct stays as it is)  */
+  int32_t autotune;        /* 1 (default): FP32 descreening sums over 64 or 128
+                              columns, whichever the first run's size settles;
+                              0: over 128.  Launch shapes follow from the sizes */
 } rstg_system_opts;
 void rstg_system_opts_default(rstg_system_opts* o);
 
@@ -323,10 +324,13 @@ rstg_status rstg_system_last_stats(const rstg_system* s, int64_t* stats4);
  * pair-kernel threads per row, its minimum resident blocks per SM (register
  * cap) on large batches, SASA warps per block, frames per batch, 0 (nothing is
  * timed), 0, number of pair-kernel candidates (0), number of SASA candidates
- * (0), Born-radius kernel threads per row, its minimum resident blocks per SM,
- * number of its candidates (0), pair-kernel form (1 warp items); ms12 zeros.
- * The shapes follow from the sizes alone, so equal inputs give equal results.
- * Either pointer may be NULL; zeros for plain-mode systems. */
+ * (0), shares of a 128-column tile that the Born-radius kernel sums apart in
+ * FP32 (1 or 2), its minimum resident blocks per SM, number of its candidates
+ * (0), pair-kernel form (1 warp items); ms12 zeros.  The shapes follow from the
+ * sizes; the shares from the size of the first run of such a system.  Systems
+ * of one process with the same device, atom counts and sphere points have the
+ * same ones, so equal inputs give equal results.  Either pointer may be NULL;
+ * zeros for plain-mode systems. */
 rstg_status rstg_system_tuning(const rstg_system* s, int32_t* shape12, double* ms12);
 
 /* Batched Poisson-Boltzmann engine of a fused PB system (no reference

@@ -30,8 +30,11 @@
 // are FP32 with an FP64 re-check of the reference expression inside a
 // +-2e-4 A^2 band, so accessible-point counts equal the reference's.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <numeric>
 
 #include "common.cuh"
@@ -214,8 +217,8 @@ __device__ __forceinline__ float box_span2(const float4& alo, const float4& ahi,
 //            SASA neighbour list and to a short list of near pairs
 //   general  words that straddle the receptor / ligand boundary or the end of
 //            the slots, or that a finite cutoff may cut
-// FP32 far sums run over the columns of a tile in order, then enter the FP64
-// sums.  The near pairs (FP64) are evaluated after the column loop by four
+// FP32 far sums run over the columns of a tile in order (of either half of it
+// where `halves`, see psi_halves), then enter the FP64 sums.  The near pairs (FP64) are evaluated after the column loop by four
 // lanes per row over the row's whole list, so lanes stay evenly loaded.
 // Every sum has a fixed order that does not depend on the number of frames.
 // Bound by instruction issue (62 % of the slots, FMA pipe 55 %).  128 frames of
@@ -245,7 +248,7 @@ __global__ void __launch_bounds__(32 * kPsiWarps, 3)
     k_psi(int nC, int nR, const float4* __restrict__ xyz32, const double* __restrict__ xyz64,
           const float4* __restrict__ boxes, const float4* __restrict__ P32, const double* __restrict__ rho64,
           const double* __restrict__ sj64, const double* __restrict__ rad64, const double* __restrict__ q64, GbConstF k,
-          int cap, int* __restrict__ nbr, int* __restrict__ nbrcnt, double* __restrict__ R64, float4* __restrict__ Rf,
+          int halves, int cap, int* __restrict__ nbr, int* __restrict__ nbrcnt, double* __restrict__ R64, float4* __restrict__ Rf,
           float* __restrict__ dRf, double* __restrict__ wdec, double* __restrict__ part, int* __restrict__ diag) {
   extern __shared__ __align__(16) unsigned char psi_raw[];
   PsiSmem& sm = *reinterpret_cast<PsiSmem*>(psi_raw);
@@ -331,8 +334,19 @@ __global__ void __launch_bounds__(32 * kPsiWarps, 3)
       const int kt = kb + q, t = tfirst + tstep * kt, j0 = t * kTile;
       if (t >= ntile) break;
       R[0].po = R[0].pc = R[1].po = R[1].pc = 0.f;
+      auto flush = [&] {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          psiO[r] += (double)R[r].po;
+          psiX[r] += (double)R[r].pc;
+        }
+      };
 #pragma unroll 1
       for (int w = 0; w < 4; w++) {
+        if (w == 2 && halves) {
+          flush();
+          R[0].po = R[0].pc = R[1].po = R[1].pc = 0.f;
+        }
         if ((w & 1) == 0) {  // stage the next half of the tile: two columns per lane
           const int j = j0 + 32 * w + 2 * lane;
           const float4 x0 = X[min(j, nC - 1)], x1 = X[min(j + 1, nC - 1)], p0 = P32[min(j, nC - 1)],
@@ -471,11 +485,7 @@ __global__ void __launch_bounds__(32 * kPsiWarps, 3)
           }
         }
       }
-#pragma unroll
-      for (int r = 0; r < 2; r++) {
-        psiO[r] += (double)R[r].po;
-        psiX[r] += (double)R[r].pc;
-      }
+      flush();
     }
   }
   __syncthreads();  // every warp is done with its columns: the union turns into the partial sums
@@ -1981,11 +1991,46 @@ void System::launch_pairs(int64_t F) {
       k2part.as<double>(), diag.as<int>());
 }
 
+// FP32 sums of k_psi over 64 columns (a tile's halves apart) or 128.  Energies
+// differ by about 1e-8 between the two, and the choice is the one that systems
+// have had since their launch shapes were timed on the first run: two threads a
+// row, 64 columns each, at four blocks of 128 rows an SM, against one thread at
+// eight.  The former won by more than 2 % where its waves counted half were
+// fewer, that is where they are odd in number (up to five; later the difference
+// is too small), except on fewer than 91 atoms and on 136 to 256 of which 4
+// blocks an SM are resident (0.96 to 1.1 of the other's time), and in a second wave
+// on 7,500 atoms and more, whose columns outlast the tail (0.94 to 0.97 from
+// 5.2 blocks an SM).  Of 235 random sizes where the timed choice repeated
+// itself this rule gives 227.
+static bool psi_halves(int64_t nC, int64_t frames, int sms) {
+  const int64_t blocks = (nC + kTile - 1) / kTile * frames, waves = (blocks + 4 * sms - 1) / (4 * sms);
+  if (waves == 1) return nC > 90 && (blocks <= 3 * sms || nC <= 135 || nC > 256);
+  if (waves == 2) return nC >= 7500 && 5 * blocks >= 26 * sms;
+  return waves == 3 || waves == 5;
+}
+
+// The choice holds for every system of the process with the same device, atom
+// counts and sphere points, so that equal inputs give equal results whatever
+// the number of frames; the first run of such a system makes it, for its batch
+// or the frames that hold 2,048 tile pairs.  Without autotune: 128.
+void System::choose_psi(int64_t F) {
+  if (psi_shares > 0) return;
+  psi_shares = 1;
+  if (!opts.autotune) return;
+  static std::mutex mu;
+  static std::map<std::array<int64_t, 4>, int> chosen;
+  const int64_t nb = (nC + kTile - 1) / kTile, pairs = nb * (nb + 1) / 2;
+  const int64_t frames = std::max<int64_t>(1, std::min(batch, std::max(std::min(F, batch), (2048 + pairs - 1) / pairs)));
+  std::lock_guard<std::mutex> lk(mu);
+  psi_shares = chosen.emplace(std::array<int64_t, 4>{ctx->device, nC, nR, fp->npts},
+                              psi_halves(nC, frames, ctx->prop.multiProcessorCount) ? 2 : 1).first->second;
+}
+
 void System::launch_psi(int64_t F) {
   FusedParams& P = *fp;
   k_psi<<<dim3((unsigned)psi_blocks(nC), (unsigned)F), 32 * kPsiWarps, sizeof(PsiSmem), stream()>>>(
       (int)nC, (int)nR, xyz32.as<float4>(), xyz64.as<double>(), boxes.as<float4>(), P.P32.as<float4>(),
-      P.rho64.as<double>(), P.sj64.as<double>(), P.rad64.as<double>(), P.q64.as<double>(), P.gb, nbr_cap, nbr.as<int>(),
+      P.rho64.as<double>(), P.sj64.as<double>(), P.rad64.as<double>(), P.q64.as<double>(), P.gb, psi_shares == 2, nbr_cap, nbr.as<int>(),
       nbrcnt.as<int>(), R64.as<double>(), Rf.as<float4>(), dRf.as<float>(), wdec.as<double>(),
       k1part.as<double>(), diag.as<int>());
 }
@@ -2005,7 +2050,7 @@ void System::launch_sasa(int64_t F, cudaStream_t st) {
 
 void System::tuning(int32_t* shape12, double* ms12) const {
   // every launch shape follows from the sizes: no candidates
-  int32_t o[12] = {1, 2, kSasaWarps, (int32_t)batch, 0, 0, 0, 0, 1, 3, 0, 1};
+  int32_t o[12] = {1, 2, kSasaWarps, (int32_t)batch, 0, 0, 0, 0, std::max(psi_shares, 1), 3, 0, 1};
   if (shape12) memcpy(shape12, o, sizeof(o));
   if (ms12)
     for (int k = 0; k < 12; k++) ms12[k] = 0.0;
@@ -2307,6 +2352,7 @@ void System::run(const void* frames, bool f64, bool host_in, int64_t F, rstg_fra
   int64_t nres = fp->nres;
   for (int attempt = 0; attempt < 3; attempt++) {
     ensure_buffers(std::min(F, batch));
+    choose_psi(F);
     RSTG_CUDA(cudaMemsetAsync(diag.p, 0, 64, st));
     last_stats[0] = 0;
     for (int64_t f0 = 0; f0 < F; f0 += batch) {

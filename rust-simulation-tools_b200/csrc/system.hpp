@@ -38,6 +38,7 @@ struct System {
   int nbr_cap = 320;
   int pairs_per_sm[2] = {};  // resident k_pairs blocks per SM of each shape (persistent grid), 0 until queried
   int sasa_warps = 4;        // warps per k_sasa block
+  int psi_shares = 0;        // shares of a 128-column tile whose FP32 sums k_psi keeps apart: 1 or 2, 0 until the first run
   void tuning(int32_t* shape12, double* ms12) const;
 
   // per-batch buffers (fused)
@@ -81,6 +82,7 @@ struct System {
   };
   void launch_batch(const void* d_frames, bool f64, int64_t F, rstg_frame_energy* d_out,
                     rstg_residue_energy* d_decomp, Prof* prof = nullptr);
+  void choose_psi(int64_t F);
   void launch_pairs(int64_t F);
   void launch_psi(int64_t F);
   void launch_sasa(int64_t F, cudaStream_t st);

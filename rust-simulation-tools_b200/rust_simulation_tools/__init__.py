@@ -789,8 +789,11 @@ class BindingSystem:
                 "neighbour_overflow": int(st[3])}
 
     def tuning(self) -> dict:
-        """Launch shapes of the fused engine.  They follow from the sizes
-        alone: ``tuned`` is false and the candidate lists are empty."""
+        """Launch shapes of the fused engine.  They follow from the sizes:
+        ``tuned`` is false and the candidate lists are empty.
+        ``psi_threads_per_row`` is the number of shares of a 128-column tile
+        whose descreening terms are summed apart in FP32, settled by the first
+        run of a system of these sizes (1 with ``autotune=False``)."""
         sh = (C.c_int32 * 12)()
         ms = np.zeros(12)
         check(N.lib.rstg_system_tuning(self._h, sh, _dp(ms)))
