@@ -1,6 +1,7 @@
 // extern "C" surface of librstg (include/rstg.h).
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <memory>
 
 #include "frame_plain.hpp"
@@ -90,25 +91,53 @@ DevBuf& DevBuf::operator=(DevBuf&& o) noexcept {
   return *this;
 }
 
-cudaStream_t Ctx::side_fork(int k) {
-  if (!own_stream || k < 1) return stream;
-  while ((int)side.size() < k) {
-    cudaStream_t w;
-    cudaEvent_t e;
-    RSTG_CUDA(cudaStreamCreateWithFlags(&w, cudaStreamNonBlocking));
-    side.push_back(w);
-    RSTG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    side_ev.push_back(e);
+SideStreams::SideStreams() {
+  try {
+    for (cudaStream_t& w : s) RSTG_CUDA(cudaStreamCreateWithFlags(&w, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&fork, &join[0], &join[1]}) RSTG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  } catch (...) {
+    release();
+    throw;
   }
-  RSTG_CUDA(cudaEventRecord(side_ev[k - 1], stream));
-  RSTG_CUDA(cudaStreamWaitEvent(side[k - 1], side_ev[k - 1], 0));
-  return side[k - 1];
 }
-void Ctx::side_join(int parts) {
-  if (!own_stream) return;
-  for (int k = 1; k < parts && k <= (int)side.size(); k++) {
-    RSTG_CUDA(cudaEventRecord(side_ev[k - 1], side[k - 1]));
-    RSTG_CUDA(cudaStreamWaitEvent(stream, side_ev[k - 1], 0));
+void SideStreams::release() {
+  for (cudaEvent_t e : {fork, join[0], join[1]})
+    if (e) cudaEventDestroy(e);
+  for (cudaStream_t w : s)
+    if (w) cudaStreamDestroy(w);
+}
+
+SideLease::SideLease(Ctx* c) : c_(c), unwinding_(std::uncaught_exceptions()) {
+  if (!c->own_stream) return;
+  {
+    std::lock_guard<std::mutex> lk(c->side_mu);
+    if (!c->side_free.empty()) {
+      set_ = std::move(c->side_free.back());
+      c->side_free.pop_back();
+    }
+  }
+  if (!set_) set_ = std::make_unique<SideStreams>();
+}
+SideLease::~SideLease() {
+  if (!set_) return;
+  if (std::uncaught_exceptions() > unwinding_)
+    for (cudaStream_t w : set_->s) cudaStreamSynchronize(w);
+  try {
+    std::lock_guard<std::mutex> lk(c_->side_mu);
+    c_->side_free.push_back(std::move(set_));
+  } catch (...) {  // no room to keep the set: it goes with the lease
+  }
+}
+void SideLease::fork() {
+  if (!set_) return;
+  RSTG_CUDA(cudaEventRecord(set_->fork, c_->stream));
+  for (cudaStream_t w : set_->s) RSTG_CUDA(cudaStreamWaitEvent(w, set_->fork, 0));
+}
+void SideLease::join() {
+  if (!set_) return;
+  for (int k = 0; k < 2; k++) {
+    RSTG_CUDA(cudaEventRecord(set_->join[k], set_->s[k]));
+    RSTG_CUDA(cudaStreamWaitEvent(c_->stream, set_->join[k], 0));
   }
 }
 
@@ -239,8 +268,7 @@ void rstg_ctx_destroy(rstg_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  for (cudaStream_t w : c->side) cudaStreamDestroy(w);
-  for (cudaEvent_t e : c->side_ev) cudaEventDestroy(e);
+  c->side_free.clear();
   if (c->own_stream) cudaStreamDestroy(c->stream);
   DevicePool& p = device_pool(c->device);
   {

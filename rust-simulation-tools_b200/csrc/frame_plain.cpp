@@ -2,7 +2,6 @@
 #include "frame_plain.hpp"
 
 #include <cmath>
-#include <exception>
 #include <unordered_map>
 
 namespace rstg {
@@ -46,26 +45,17 @@ void PlainFrameEval::set_coords(const double* xc, std::vector<double>& hx) {
     RSTG_CUDA(cudaMemcpyAsync(xyz.p, hx.data(), hx.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
 }
 
-// A call that throws between fork and join leaves no kernel running on memory
-// that its buffers give back to the pool.
-struct SideGuard {
-  Ctx* ctx;
-  ~SideGuard() {
-    if (std::uncaught_exceptions() > 0)
-      for (cudaStream_t w : ctx->side) cudaStreamSynchronize(w);
-  }
-};
-
 rstg_frame_energy PlainFrameEval::run(const double* xc) {
   cudaStream_t st = ctx->stream;
-  SideGuard guard{ctx};
+  SideLease side(ctx);
   std::vector<double> hx;
   set_coords(xc, hx);
   RSTG_CUDA(cudaMemsetAsync(overflow.p, 0, 8, st));
   RSTG_CUDA(cudaMemsetAsync(out.p, 0, 36 * 8, st));
   double* o = out.as<double>();
   // the three terms beside one another (a term of a few thousand atoms leaves the GPU partly idle)
-  cudaStream_t s1 = ctx->side_fork(1), s2 = ctx->side_fork(2);
+  side.fork();
+  const cudaStream_t s1 = side[0], s2 = side[1];
   for (int k = 0; k < 3; k++) {
     const DevTopo& d = sub[k].dev;
     plain_mm_energy(ctx, st, d, coords(k), o + 12 * k);
@@ -76,7 +66,7 @@ rstg_frame_energy PlainFrameEval::run(const double* xc) {
     plain_sasa(ctx, s2, d, coords(k), sa.probe_radius, n_sphere, sphere.as<double>(), per_atom[k].as<double>(),
                o + 12 * k + 8, overflow.as<int>());
   }
-  ctx->side_join(3);
+  side.join();
   double h[36];
   int ov = 0;
   RSTG_CUDA(cudaMemcpyAsync(h, out.p, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -114,11 +104,12 @@ void PlainFrameEval::decompose(const double* xc, const rstg_gb_params& gb, rstg_
   std::vector<double> hx;
   set_coords(xc, hx);
   DevBuf rows(std::max<int64_t>(nr, 1) * 16, st), cols(std::max<int64_t>(nl, 1) * 16, st), tot(3 * 2 * 8, st);
-  SideGuard guard{ctx};
+  SideLease side(ctx);
   RSTG_CUDA(cudaMemsetAsync(tot.p, 0, 48, st));
   RSTG_CUDA(cudaMemsetAsync(overflow.p, 0, 8, st));
   // pairs, GB and SA beside one another (decomposition.rs:295-307, 355-363)
-  cudaStream_t s1 = ctx->side_fork(1), s2 = ctx->side_fork(2);
+  side.fork();
+  const cudaStream_t s1 = side[0], s2 = side[1];
   plain_decomp_pairs(ctx, st, sub[0].dev, coords(0), rec_idx.as<int>(), (int)nr, lig_idx.as<int>(), (int)nl,
                      rows.as<double>(), cols.as<double>());
   for (int k = 0; k < 3; k++) {
@@ -129,7 +120,7 @@ void PlainFrameEval::decompose(const double* xc, const rstg_gb_params& gb, rstg_
     plain_sasa(ctx, s2, d, coords(k), sa.probe_radius, n_sphere, sphere.as<double>(), per_atom[k].as<double>(),
                tot.as<double>() + 2 * k + 1, overflow.as<int>());
   }
-  ctx->side_join(3);
+  side.join();
   std::vector<double> hr(2 * nr), hc(2 * nl), ht(6), hR[3], hS[3];
   for (int k = 0; k < 3; k++) {
     int64_t n = sub[k].dev.n;

@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -99,6 +100,17 @@ struct DevBuf {
   }
 };
 
+// Two streams beside a context's own one and the events that order them.
+struct SideStreams {
+  cudaStream_t s[2] = {};
+  cudaEvent_t fork = nullptr, join[2] = {};
+  SideStreams();
+  ~SideStreams() { release(); }
+  void release();
+  SideStreams(const SideStreams&) = delete;
+  SideStreams& operator=(const SideStreams&) = delete;
+};
+
 struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -106,14 +118,31 @@ struct Ctx {
   std::recursive_mutex mu;
   std::atomic<int64_t> launches{0};
   cudaDeviceProp prop{};
-  // Streams beside the context's own one, for independent parts of one call
-  // (under mu; empty where the caller owns the stream, since every kernel then
-  // runs on it): side_fork orders them after the stream, side_join the stream after them.
-  std::vector<cudaStream_t> side;
-  std::vector<cudaEvent_t> side_ev;
-  cudaStream_t side_fork(int k);  // stream of part k >= 1 (the stream itself where there are none)
-  void side_join(int parts);
+  std::mutex side_mu;
+  std::vector<std::unique_ptr<SideStreams>> side_free;  // sets that no call holds (under side_mu)
   void bind() const { cudaSetDevice(device); }
+};
+
+// Side streams for independent parts of one call, held by that call alone:
+// calls of one context run at the same time from several threads (systems in
+// plain mode, a server's workers), and an event recorded anew by another call
+// would unorder this one's kernels.  Where the caller owns the stream every part
+// runs on it.  A call that throws between fork and join leaves no kernel running
+// on memory that its buffers give back to the pool: declare the lease after them.
+class SideLease {
+ public:
+  explicit SideLease(Ctx* c);
+  ~SideLease();
+  SideLease(const SideLease&) = delete;
+  SideLease& operator=(const SideLease&) = delete;
+  void fork();  // both streams after what the context's stream holds
+  void join();  // the context's stream after both
+  cudaStream_t operator[](int k) const { return set_ ? set_->s[k] : c_->stream; }
+
+ private:
+  Ctx* c_;
+  int unwinding_;
+  std::unique_ptr<SideStreams> set_;
 };
 
 // Records a kernel launch for the context's counter and checks the launch.
