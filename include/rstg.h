@@ -337,7 +337,9 @@ rstg_status rstg_system_tuning(const rstg_system* s, int32_t* shape12, double* m
  * counterpart), accumulated over runs: grids solved, lock-step multigrid
  * cycles, grids solved by the FP64 path, then host milliseconds of the
  * set-up (maps, boundary values), the cycles and the finish (fallbacks,
- * energies).  Eight doubles; zeros for GB systems. */
+ * energies); of the last solve, the priority of its stream and the least urgent
+ * priority among the streams its cycles ran on.  Eight doubles; zeros for GB
+ * systems. */
 rstg_status rstg_system_pb_stats(const rstg_system* s, double* stats8);
 /* Frames per batched PB launch sequence (0: from the device memory budget,
  * at most 60 % of the free memory and 64 GB, about 140 bytes per grid point

@@ -153,6 +153,8 @@ rstg_status rstg_system_pb_stats(const rstg_system* s, double* o) {
     o[3] = t.ms_setup;
     o[4] = t.ms_cycles;
     o[5] = t.ms_finish;
+    o[6] = t.priority;
+    o[7] = t.chain_priority;
   });
 }
 

@@ -1517,11 +1517,22 @@ void PbBatchEngine::release() {
   for (DevBuf& b : chain_lists_) b = DevBuf();
 }
 
+// A chain's stream has the priority of the solve's own: a server gives each chunk
+// a stream of its request's rank, and the solve waits for every chain at the
+// end of a chunk of cycles.  Nothing is pending on the streams between solves.
 cudaStream_t PbBatchEngine::chain_stream(int k) {
-  if (!chain_streams_[k]) {
-    RSTG_CUDA(cudaStreamCreateWithFlags(&chain_streams_[k], cudaStreamNonBlocking));
-    RSTG_CUDA(cudaEventCreateWithFlags(&chain_join_[k], cudaEventDisableTiming));
+  int want = 0;
+  RSTG_CUDA(cudaStreamGetPriority(st_, &want));
+  if (chain_streams_[k]) {
+    int have = 0;
+    RSTG_CUDA(cudaStreamGetPriority(chain_streams_[k], &have));
+    if (have != want) {
+      RSTG_CUDA(cudaStreamDestroy(chain_streams_[k]));
+      chain_streams_[k] = nullptr;
+    }
   }
+  if (!chain_streams_[k]) RSTG_CUDA(cudaStreamCreateWithPriority(&chain_streams_[k], cudaStreamNonBlocking, want));
+  if (!chain_join_[k]) RSTG_CUDA(cudaEventCreateWithFlags(&chain_join_[k], cudaEventDisableTiming));
   return chain_streams_[k];
 }
 
@@ -1985,7 +1996,14 @@ void PbBatchEngine::solve(std::vector<PbJob>& jobs, const rstg_pb_params& p, con
   auto chain_of = [&](int j) -> Chain& {  // one chain in a profiled run: launches one after another, bytes a launch of all grids
     return chains[profile ? 0 : (jobs[j].uniform ? 1 : 0) + 2 * ((j >> 1) % (kChains / 2))];
   };
-  for (int k = 0; k < kChains; k++) chains[k].s = k && !profile ? chain_stream(k) : st;
+  RSTG_CUDA(cudaStreamGetPriority(st, &stats.priority));
+  stats.chain_priority = stats.priority;
+  for (int k = 0; k < kChains; k++) {
+    int prio = 0;
+    chains[k].s = k && !profile ? chain_stream(k) : st;
+    RSTG_CUDA(cudaStreamGetPriority(chains[k].s, &prio));
+    stats.chain_priority = std::max(stats.chain_priority, prio);
+  }
   // profile mode: events around every launch; the level-0 kernels also
   // carry their algorithmic bytes (compulsory DRAM traffic per launch) from
   // the current lists.  kind: roofline slot (-1 none); det: kernel family.

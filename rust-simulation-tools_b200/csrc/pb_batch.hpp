@@ -34,6 +34,8 @@ struct PbBatchStats {
   double ms_setup = 0.0;   // maps and boundary values
   double ms_cycles = 0.0;  // lock-step multigrid cycles
   double ms_finish = 0.0;  // FP64 fallbacks, energies
+  int priority = 0;        // priority of the last solve's stream
+  int chain_priority = 0;  // the least urgent priority its launches had
 };
 
 // Per-kernel device time of the level-0 multigrid kernels (profile mode):
