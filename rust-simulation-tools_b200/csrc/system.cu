@@ -28,7 +28,7 @@
 // (r < 3.5 A for LJ/Coulomb, any pair outside the far-field series domain for
 // the HCT integral) take the reference's FP64 expressions; SASA point tests
 // are FP32 with an FP64 re-check of the reference expression inside a
-// +-2e-4 A^2 band, so accessible-point counts equal the reference's.
+// band of +-2e-4 A^2 (more for large probes), so accessible-point counts equal the reference's.
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -43,10 +43,11 @@
 
 namespace rstg {
 
-// A^2: ten times the FP32 error bound of a point-to-neighbour squared distance
-// at these coordinates; SASA point tests closer than this to the threshold are
-// redone in FP64 with the reference's rounding
-static constexpr float kSasaBand = 2e-4f;
+// A^2: SASA point tests closer than this to the threshold are redone in FP64 with
+// the reference's rounding.  A test's FP32 error grows with the squared reach
+// (er + the largest expanded radius)^2, the bound of its terms: 4e-6 of it is ten
+// times the error, 2e-4 at a probe of 1.4 A.
+static constexpr float kSasaBand = 2e-4f, kSasaBandRel = 4e-6f;
 static constexpr float kNbGuard2 = 3.5f * 3.5f;
 
 // k_sasa: warps per block (fewer where the neighbours of four do not fit), and classes of its neighbour order per part (own, other)
@@ -74,6 +75,7 @@ struct FusedParams {
       res_ptr, res_slots, bterms, bpar, corr;
   int nt = 0, nb = 0, nitems = 0, nrec = 0, npts = 0, nres = 0, nterms = 0, ncorr = 0;
   double probe = 1.4;
+  float max_ext = 0.f;  // largest radius + probe
   GbConstF gb{};
 };
 
@@ -1059,8 +1061,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // where g = s . 2 er v - (er^2 + |v|^2 - ro^2) > 0, v the vector to j and ro
 // its expanded radius: three multiply-adds a test instead of a distance.  v is
 // the difference of the FP64 coordinates, rounded once, so |g| errs by less
-// than a tenth of kSasaBand; points whose largest g falls inside the band are
-// decided with the reference's FP64 expression, so the counts are the
+// than a tenth of the band (kSasaBand); points whose largest g falls inside the
+// band are decided with the reference's FP64 expression, so the counts are the
 // reference's.  Neighbours are ordered own part first, then the other part,
 // each by the part of the sphere that it buries (the cap's cosine, in classes;
 // a counting sort), so that buried points, nearly all of them, finish after a
@@ -1075,7 +1077,7 @@ template <int SPLIT>
 __global__ void __launch_bounds__(32 * kSasaWarps)
     k_sasa(int nC, int nR, int cap, const int* __restrict__ nbr, const int* __restrict__ nbrcnt,
            const float4* __restrict__ P32, const double* __restrict__ xyz64, const double* __restrict__ rad64,
-           double probe, int npts, const float4* __restrict__ sph32, const double* __restrict__ sph64,
+           double probe, float max_ext, int npts, const float4* __restrict__ sph32, const double* __restrict__ sph64,
            double* __restrict__ sasa, int* __restrict__ diag) {
   extern __shared__ __align__(16) unsigned char sasa_raw[];
   __shared__ int2 counts[kSasaWarps];
@@ -1096,7 +1098,8 @@ __global__ void __launch_bounds__(32 * kSasaWarps)
     const double x0 = X64[3 * i], y0 = X64[3 * i + 1], z0 = X64[3 * i + 2];
     const bool in_r = i < nR;
     er = rad64[i] + probe;
-    const float erf = (float)er, er2 = erf * erf, inv2er = 4.f / erf;
+    const float erf = (float)er, er2 = erf * erf, inv2er = 4.f / erf, reach = erf + max_ext;
+    const float band = fmaxf(kSasaBand, kSasaBandRel * reach * reach);
     if (lane < 2 * kSasaBins) hist[lane] = 0;
     __syncwarp();
     // a neighbour's vector (of the FP64 coordinates, rounded once), constant term and class
@@ -1187,14 +1190,14 @@ __global__ void __launch_bounds__(32 * kSasaWarps)
         m0 = max3(m0, u, v);
         un2(fma2(qx, x.y, fma2(qy, y.y, fma2(qz, z.y, c.y))), u, v);
         m1 = max3(m1, u, v);
-        if (__all_sync(0xffffffffu, fminf(m0, m1) > kSasaBand)) break;
+        if (__all_sync(0xffffffffu, fminf(m0, m1) > band)) break;
       }
     };
     // a point whose largest g lies in the band: the reference's test of the neighbours in the band
     auto decide = [&](const float4& p, int a, int b) {
       for (int k = a; k < b; k++) {
         const float g = fmaf(p.x, wx[k], fmaf(p.y, wy[k], fmaf(p.z, wz[k], wc[k])));
-        if (g < -2.f * kSasaBand) continue;
+        if (g < -2.f * band) continue;
         rechecks++;
         const int j = val[k];
         if (exact_buried(X64, i, j, sph64, __float_as_int(p.w), er, __dadd_rn(rad64[j], probe))) return true;
@@ -1202,7 +1205,7 @@ __global__ void __launch_bounds__(32 * kSasaWarps)
       return false;
     };
     auto buried = [&](const float4& p, float m, int a, int b) {
-      return m > kSasaBand || (m >= -kSasaBand && decide(p, a, b));
+      return m > band || (m >= -band && decide(p, a, b));
     };
     // sph32 is stored patch by patch (32 points compact on the sphere per
     // patch); .w holds the point's index in the reference's order
@@ -1243,7 +1246,7 @@ __global__ void __launch_bounds__(32 * kSasaWarps)
     sasa[2 * o + 1] = ((double)cs / (double)npts) * area;  // in its own part
   }
 }
-using SasaFn = void (*)(int, int, int, const int*, const int*, const float4*, const double*, const double*, double, int,
+using SasaFn = void (*)(int, int, int, const int*, const int*, const float4*, const double*, const double*, double, float, int,
                         const float4*, const double*, double*, int*);
 static const SasaFn kSasaFn[3] = {k_sasa<1>, k_sasa<2>, k_sasa<4>};
 
@@ -1861,6 +1864,7 @@ void System::prepare_fused(const double* x0) {
       sm = std::max(sm, std::fabs((double)P[a].z));
       rm = std::max(rm, std::fabs((double)P[a].y));
     }
+    F.max_ext = (float)ext;
     const double far2 = std::max({4.0 * ext * ext * 1.00001 + 1e-4, 16.0 * sm * sm, (rm + sm) * (rm + sm)});
     k.tile_far2 = (float)(far2 * 1.001 + 0.01);
   }
@@ -2044,7 +2048,7 @@ void System::launch_sasa(int64_t F, cudaStream_t st) {
   kSasaFn[lg]<<<dim3((unsigned)((nC + per - 1) / per), (unsigned)F), 32 * sasa_warps,
                 sasa_smem(nbr_cap, sasa_warps), st>>>(
       (int)nC, (int)nR, nbr_cap, nbr.as<int>(), nbrcnt.as<int>(), P.P32.as<float4>(), xyz64.as<double>(),
-      P.rad64.as<double>(), P.probe, P.npts, P.sphere32.as<float4>(), P.sphere64.as<double>(), sasa.as<double>(),
+      P.rad64.as<double>(), P.probe, P.max_ext, P.npts, P.sphere32.as<float4>(), P.sphere64.as<double>(), sasa.as<double>(),
       diag.as<int>());
 }
 
