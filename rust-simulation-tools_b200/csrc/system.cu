@@ -676,7 +676,7 @@ template <bool kSalt>
 constexpr float kMmScale = kSalt ? -0.5f : 1.f;
 
 // Columns [lo, hi) of the word from slot j0 on one by one, with every test: the receptor /
-// ligand class of each pair, the cutoff, the exclusion (wex) and 1-4 (w14)
+// ligand class of each pair, the cutoff (of the GB terms), the exclusion (wex) and 1-4 (w14)
 // masks.  Cross pairs contribute the complex GB energy only (their
 // Lennard-Jones, Coulomb and binding GB terms are summed in FP64 by
 // k_rl_rows).  FP64 Lennard-Jones / Coulomb pairs are marked in dfr.  fused
@@ -691,22 +691,26 @@ __device__ __forceinline__ void pair_word(int lo, int hi, int j0, int nR, bool f
   for (int jj = lo; jj < hi; jj++) {
     const float dx = P.xi.x - T.x[jj], dy = P.xi.y - T.y[jj], dz = P.xi.z - T.z[jj];
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    if (r2 > k.fcut2) continue;
+    const bool same = (j0 + jj < nR) == P.in_r;
     const float qq = P.xi.w * T.q[jj];
-    const float tc = r2 * P.iRc * T.iRc[jj];  // -t log2(e): P.iRc carries -log2(e) / (4 R_C,i)
-    const float RRc = P.Ri.x * T.Rc[jj];
-    float eC, f2C, finvC, EC;
-    const float wC = gb_pair_parts(qq, r2, RRc, tc, k, eC, f2C, finvC, EC), pC = __fmul_rn(wC, finvC);
-    a.c = fused ? fmaf(wC, finvC, a.c) : __fadd_rn(a.c, pC);
-    if ((j0 + jj < nR) != P.in_r) continue;
-    const float ts = r2 * P.iRs * T.iRs[jj];
-    const float dRR = fmaf(P.Ri.x, T.dR[jj], T.Rs[jj] * P.dRi);  // RcRc' - RsRs'
-    const float dp = (dRR == 0.f || (tc <= kU16 && ts <= kU16))
-                         ? 0.f
-                         : gb_pair_delta(qq, r2, RRc, P.Ri.y * T.Rs[jj], P.iRsN * T.iRs[jj], dRR, tc, ts, eC, f2C, finvC,
-                                         EC, k);
-    a.s = __fadd_rn(a.s, __fsub_rn(pC, dp));
-    a.d = __fadd_rn(a.d, dp);
+    if (!(r2 > k.fcut2)) {  // the cutoff is of the GB terms alone
+      const float tc = r2 * P.iRc * T.iRc[jj];  // -t log2(e): P.iRc carries -log2(e) / (4 R_C,i)
+      const float RRc = P.Ri.x * T.Rc[jj];
+      float eC, f2C, finvC, EC;
+      const float wC = gb_pair_parts(qq, r2, RRc, tc, k, eC, f2C, finvC, EC), pC = __fmul_rn(wC, finvC);
+      a.c = fused ? fmaf(wC, finvC, a.c) : __fadd_rn(a.c, pC);
+      if (same) {
+        const float ts = r2 * P.iRs * T.iRs[jj];
+        const float dRR = fmaf(P.Ri.x, T.dR[jj], T.Rs[jj] * P.dRi);  // RcRc' - RsRs'
+        const float dp = (dRR == 0.f || (tc <= kU16 && ts <= kU16))
+                             ? 0.f
+                             : gb_pair_delta(qq, r2, RRc, P.Ri.y * T.Rs[jj], P.iRsN * T.iRs[jj], dRR, tc, ts, eC, f2C,
+                                             finvC, EC, k);
+        a.s = __fadd_rn(a.s, __fsub_rn(pC, dp));
+        a.d = __fadd_rn(a.d, dp);
+      }
+    }
+    if (!same) continue;
     const bool is14 = (w14 >> jj) & 1u, excl = (wex >> jj) & 1u;
     if (is14 || (!excl && r2 < kNbGuard2)) {
       dfr |= 1u << jj;
@@ -726,10 +730,11 @@ __device__ __forceinline__ void pair_word(int lo, int hi, int j0, int nR, bool f
 // complex radii only, see pair_word); kSmall words whose radii differ too little for |tC - tS| >= 0.2, so
 // the difference form needs its common branch only (a pair with t beyond 16
 // for one radii set alone counts as beyond it for both: below 1e-9 of the
-// pair); kAny words that evaluate both branches.  kTests: words that may hold
+// pair); kAny words that evaluate both branches; kMm words wholly beyond the
+// cutoff, Lennard-Jones and Coulomb terms alone.  kTests: words that may hold
 // FP64 Lennard-Jones / Coulomb pairs or masked ones.  No cutoff test: the
 // caller has ruled it out.
-enum PairForm { kCross, kCrossFused, kSmall, kAny };
+enum PairForm { kCross, kCrossFused, kSmall, kAny, kMm };
 template <bool kSalt, PairForm kForm, bool kTests>
 __device__ __forceinline__ void pair_word2(const PairRow& P, const GbConstF& k, const PairTile& T,
                                            const float2* __restrict__ slj, unsigned wex, unsigned w14, PairSum& a,
@@ -739,10 +744,33 @@ __device__ __forceinline__ void pair_word2(const PairRow& P, const GbConstF& k, 
            dRi = dup2(P.dRi);
   const f2 fie = dup2(k.fie), nfio = dup2(-k.fio), fkl = dup2(k.fkl), fk = dup2(k.fk);
   const unsigned skip = wex | w14;
+  // Lennard-Jones and Coulomb terms of two columns
+  auto mm = [&](f2 r2, f2 qq, int t0, int t1, int b) {
+    float r0, r1, i0, i1, q0, q1;
+    un2(r2, r0, r1);
+    const f2 ri = pk2(rsqrtf(r0), rsqrtf(r1)), i2 = mul2(ri, ri);
+    un2(mul2(mul2(i2, i2), i2), i0, i1);
+    un2(mul2(qq, ri), q0, q1);
+    const float2 A = slj[t0 + P.ti], B = slj[t1 + P.ti];
+    const float m0 = fmaf(A.x * i0, i0, fmaf(-A.y, i0, q0)), m1 = fmaf(B.x * i1, i1, fmaf(-B.y, i1, q1));
+    if (kTests) {
+      const unsigned o0 = 1u << b, o1 = 2u << b;
+      if (r0 < kNbGuard2) dfr |= o0;
+      if (r1 < kNbGuard2) dfr |= o1;
+      if (!((dfr | skip) & o0)) a.m = __fadd_rn(a.m, m0);
+      if (!((dfr | skip) & o1)) a.m = __fadd_rn(a.m, m1);
+    } else {
+      a.m = __fadd_rn(__fadd_rn(a.m, m0), m1);
+    }
+  };
   auto two = [&](f2 x, f2 y, f2 z, f2 q, f2 Rc, f2 Rs, f2 iRc, f2 iRs, f2 dR, int t0, int t1, int b) {
     const f2 dx = sub2(xi, x), dy = sub2(yi, y), dz = sub2(zi, z);
     const f2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
     const f2 qq = mul2(qi, q), tc = mul2(mul2(r2, iRci), iRc), RRc = mul2(Rci, Rc);
+    if (kForm == kMm) {
+      mm(r2, qq, t0, t1, b);
+      return;
+    }
     float u0, u1;
     un2(tc, u0, u1);
     const bool v0 = u0 > kU16, v1 = u1 > kU16;
@@ -814,22 +842,7 @@ __device__ __forceinline__ void pair_word2(const PairRow& P, const GbConstF& k, 
     un2(add2(pC, nd), s0, s1);
     a.s = __fadd_rn(__fadd_rn(a.s, s0), s1);
     a.d = __fsub_rn(__fsub_rn(a.d, n0), n1);
-    float r0, r1, i0, i1, q0, q1;
-    un2(r2, r0, r1);
-    const f2 ri = pk2(rsqrtf(r0), rsqrtf(r1)), i2 = mul2(ri, ri);
-    un2(mul2(mul2(i2, i2), i2), i0, i1);
-    un2(mul2(qq, ri), q0, q1);
-    const float2 A = slj[t0 + P.ti], B = slj[t1 + P.ti];
-    const float m0 = fmaf(A.x * i0, i0, fmaf(-A.y, i0, q0)), m1 = fmaf(B.x * i1, i1, fmaf(-B.y, i1, q1));
-    if (kTests) {
-      const unsigned o0 = 1u << b, o1 = 2u << b;
-      if (r0 < kNbGuard2) dfr |= o0;
-      if (r1 < kNbGuard2) dfr |= o1;
-      if (!((dfr | skip) & o0)) a.m = __fadd_rn(a.m, m0);
-      if (!((dfr | skip) & o1)) a.m = __fadd_rn(a.m, m1);
-    } else {
-      a.m = __fadd_rn(__fadd_rn(a.m, m0), m1);
-    }
+    mm(r2, qq, t0, t1, b);
   };
 #pragma unroll 1
   for (int jj = 0; jj < 32; jj += 4) {
@@ -941,7 +954,9 @@ __global__ void __launch_bounds__(32 * kPairWarps, MINB)
       __syncwarp();
       const float4 clo = B[2 * cch], chi = B[2 * cch + 1];
       const bool cR = j0 + 32 <= nR, cL = j0 >= nR;
-      const bool packed = cch != rch && (cR || cL) && j0 + 32 <= nC && box_span2(rlo, rhi, clo, chi) * 1.0001f < k.fcut2;
+      const bool whole = cch != rch && (cR || cL) && j0 + 32 <= nC;
+      const float gap2 = box_gap2(rlo, rhi, clo, chi) * 0.9999f;
+      const bool packed = whole && box_span2(rlo, rhi, clo, chi) * 1.0001f < k.fcut2;
       const bool same = cR == in_r;  // of a packed word
       const int t0 = (rch >> 2) * kTile, u0 = (cch >> 2) * kTile;  // first slots of the row's and the column's tile
       const bool fused = (t0 + kTile <= nR && u0 >= nR) || (t0 >= nR && u0 + kTile <= nR);
@@ -956,7 +971,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, MINB)
             pair_word2<kSalt, kCrossFused, false>(P, k, T, slj, 0u, 0u, a, dfr);
           else
             pair_word2<kSalt, kCross, false>(P, k, T, slj, 0u, 0u, a, dfr);
-        else if (box_gap2(rlo, rhi, clo, chi) * 0.9999f > kNbGuard2 && !__any_sync(0xffffffffu, (mex | m14) != 0u))
+        else if (gap2 > kNbGuard2 && !__any_sync(0xffffffffu, (mex | m14) != 0u))
           if (small)
             pair_word2<kSalt, kSmall, false>(P, k, T, slj, 0u, 0u, a, dfr);
           else
@@ -967,6 +982,15 @@ __global__ void __launch_bounds__(32 * kPairWarps, MINB)
         if (!same) {
           a.s = a.d = a.m = 0.f;
           dfr = 0u;
+        }
+      }
+      if (whole && gap2 > fmaxf(k.fcut2, kNbGuard2)) {  // every pair beyond the cutoff
+        if (!__any_sync(0xffffffffu, same && live)) {
+          single = false;
+        } else if (!__any_sync(0xffffffffu, (mex | m14) != 0u)) {
+          pair_word2<kSalt, kMm, false>(P, k, T, slj, 0u, 0u, a, dfr);
+          if (!same) a.m = 0.f;
+          single = false;
         }
       }
       if (single && live) {
