@@ -65,6 +65,7 @@ struct GbConstF {
   double f0;        // -(1/eps_in - 1/eps_out)/2 without salt: the decomposition's weights (decomposition.rs:320-337)
   float fk, fie, fio, fdns, fcut2;
   float fkl;        // -fk log2(e): E = 2^(fkl f)
+  float fdev;       // 0.52 fk times the largest radius
   float tile_far2;  // A^2: k_psi row and column groups whose boxes are farther apart hold no SASA neighbours and only far-field pairs
   int no_salt, model;
   double rgbmax;
@@ -604,10 +605,10 @@ __device__ __forceinline__ float gb_pair_parts(float qq, float r2, float RiRj, f
   return -0.5f * qq * fmaf(-E, k.fio, k.fie);
 }
 
-// exp(x) - 1 without cancellation for |x| < 0.2: Taylor to x^6 (relative
-// error below x^6 / 5040 < 1.3e-8), and to x^4 where |x| < 0.1 is known
-// (relative error below x^4 / 120 < 1e-6 of a term that is itself a small
-// correction).
+// exp(x) - 1 without cancellation: for |x| < 0.2 the Taylor sum to x^6 (the
+// relative error is about x^6 / 5040 < 1.3e-8), for |x| < kSmallX that to x^4
+// (about x^4 / 120 < 9e-7 of a term that is itself a correction).
+constexpr float kSmallX = 0.1f;
 __device__ __forceinline__ float expm1_6(float x) {
   return x * (1.f + x * (0.5f + x * (1.f / 6.f + x * (1.f / 24.f + x * (1.f / 120.f + x * (1.f / 720.f))))));
 }
@@ -617,7 +618,8 @@ __device__ __forceinline__ float expm1_4(float x) { return x * (1.f + x * (0.5f 
 // differences themselves so that its rounding is relative to the difference,
 // not to p: dRR = RcRc' - RsRs' comes from the FP64 radius differences;
 // exp(-tS) = exp(-tC) (1 + expm1(tC - tS)) with tC - tS = -tC dRR / RRs;
-// 1/fC - 1/fS = -(fC - fS)/(fC fS); E/f likewise through expm1.  eC, f2C,
+// 1/fC - 1/fS = -(fC - fS)/(fC fS); E/f likewise through expm1, or as the
+// difference itself where the exponents are kSmallX and more apart.  eC, f2C,
 // finvC, EC are the complex pair's ingredients; uC, uS the base-2 exponents
 // -tC log2(e), -tS log2(e); iRRsN = ln(2) / RRs, so tC - tS = uC dRR iRRsN.
 __device__ __forceinline__ float gb_pair_delta(float qq, float r2, float RRc, float RRs, float iRRsN, float dRR,
@@ -636,7 +638,9 @@ __device__ __forceinline__ float gb_pair_delta(float qq, float r2, float RRc, fl
   float df = __fdividef(g, f2C * finvC + f2S * finvS);  // fC - fS
   float dinv = -df * finvC * finvS;                     // 1/fC - 1/fS
   if (k.no_salt) return k.fdns * qq * dinv;
-  float dh = EC * (dinv - expm1_4(k.fk * df) * finvS);  // EC/fC - ES/fS
+  const float zz = k.fk * df;
+  const float dh = fabsf(zz) < kSmallX ? EC * (dinv - expm1_4(zz) * finvS)  // EC/fC - ES/fS
+                                       : EC * finvC - ex2_approx(k.fkl * (f2S * finvS)) * finvS;
   return -0.5f * qq * (k.fie * dinv - k.fio * dh);
 }
 
@@ -727,8 +731,8 @@ __device__ __forceinline__ void pair_word(int lo, int hi, int j0, int nR, bool f
 // The word's 32 columns, two per packed instruction, each pair with the
 // scalar code's operations and rounding and the columns added in order.
 // kForm: kCross, kCrossFused receptor x ligand words (GB pair energy with
-// complex radii only, see pair_word); kSmall words whose radii differ too little for |tC - tS| >= 0.2, so
-// the difference form needs its common branch only (a pair with t beyond 16
+// complex radii only, see pair_word); kSmall words whose radii differ too little for |tC - tS| >= 0.2 and
+// for |0.73 kappa (fC - fS)| >= kSmallX, so the difference form needs its common branch only (a pair with t beyond 16
 // for one radii set alone counts as beyond it for both: below 1e-9 of the
 // pair); kAny words that evaluate both branches; kMm words wholly beyond the
 // cutoff, Lennard-Jones and Coulomb terms alone.  kTests: words that may hold
@@ -833,7 +837,18 @@ __device__ __forceinline__ void pair_word2(const PairRow& P, const GbConstF& k, 
       h = fma2(zz, h, dup2(0.5f));
       h = fma2(zz, h, dup2(1.f));
       h = mul2(zz, h);
-      const f2 ndh = mul2(E, fma2(h, finvS, D));
+      f2 ndh = mul2(E, fma2(h, finvS, D));
+      if (kForm == kAny) {
+        float z0, z1;
+        un2(zz, z0, z1);
+        if (__any_sync(0xffffffffu, fmaxf(fabsf(z0), fabsf(z1)) >= kSmallX)) {
+          float h0, h1, v0_, v1_;
+          un2(mul2(fkl, mul2(f2S, finvS)), h0, h1);
+          un2(fma2(pk2(ex2_approx(h0), ex2_approx(h1)), finvS, mul2(mul2(dup2(-1.f), E), finv)), h0, h1);
+          un2(ndh, v0_, v1_);
+          ndh = pk2(fabsf(z0) < kSmallX ? v0_ : h0, fabsf(z1) < kSmallX ? v1_ : h1);
+        }
+      }
       nd = mul2(w, fma2(fie, D, mul2(nfio, ndh)));
     } else {
       nd = mul2(w, D);
@@ -964,8 +979,10 @@ __global__ void __launch_bounds__(32 * kPairWarps, MINB)
       unsigned dfr = 0u;
       bool single = !packed;
       if (packed) {
-        // |tC - tS| = tC |RcRc' - RsRs'| / RsRs' with tC < 16
-        const bool small = 16.1f * (rdev + (1.f + rdev) * cdev) < 0.2f;
+        // |tC - tS| = tC dev, dev = |RcRc' - RsRs'| / RsRs' and tC < 16; then |fC^2 - fS^2| <= 1.01 RsRs' dev
+        // (e^-t (1 + 1.11 t) stays below 1.01) and f >= sqrt(RR), so |fC - fS| <= 0.52 R dev of the largest R
+        const float dev = rdev + (1.f + rdev) * cdev;
+        const bool small = 16.1f * dev < 0.2f && k.fdev * dev < kSmallX;
         if (!__any_sync(0xffffffffu, same && live))
           if (fused)
             pair_word2<kSalt, kCrossFused, false>(P, k, T, slj, 0u, 0u, a, dfr);
@@ -1894,6 +1911,7 @@ void System::prepare_fused(const double* x0) {
   }
   k.model = g.model;
   k.rgbmax = g.rgbmax;
+  k.fdev = 0.52f * k.fk * (float)std::min(std::fabs(g.rgbmax), 1e30);
   // neighbour capacity from the first frame (x1.5 + 32 margin; re-sized on overflow)
   {
     double cell = 0.0;
