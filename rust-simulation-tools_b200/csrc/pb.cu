@@ -1726,50 +1726,51 @@ struct PbSide {
   SolveOut* out = nullptr;
   double energy = 0.0;
 };
-// Up to this many points the two solves of a pair run side by side: one alone
-// leaves the GPU waiting at barriers (a pass over fewer points than this takes
-// less than ten barriers), and the second set of maps costs at most 130 MB.
+// Grids of up to this many points have the two solves of a pair side by side:
+// one alone leaves the GPU waiting at barriers (a pass over fewer points than
+// this takes less than ten barriers), and the second set of maps and levels costs
+// at most 140 MB.  Decided for the coarse and the fine grid apart: the
+// coarse one can be the larger (fillratio / fscale set its size).
 constexpr size_t kPairPoints = 2u << 20;
 
-// pb_solve_with_focusing, pb_energy.rs:134-322, for one or two sides on the same grids
+// pb_solve_with_focusing, pb_energy.rs:134-322, for the two sides of a pair
 static void solve_focus(Ctx* c, const Maps& fine_rho, const PbGeom* cg, const AtomsDev& A, const rstg_pb_params& p,
-                        double kap, PbSide* side, int n, double rtol) {
+                        double kap, PbSide (&side)[2], double rtol) {
   const double ein = p.solute_dielectric;
   BcSpec dh[2], bc[2];
-  for (int k = 0; k < n; k++) {
+  for (int k = 0; k < 2; k++) {
     dh[k].kind = 1;
     dh[k].kappa = side[k].ionic ? kap : 0.0;
     dh[k].eout = side[k].eout;
     bc[k] = dh[k];
   }
-  auto maps = [&](Maps& M, const PbSide& s) {
-    dielectric_maps(c, M, A, p.probe_radius, ein, s.eout);
-    kappa_map(c, M, A, p.ion_radius, kap, p.solvent_dielectric, s.ionic);
-  };
-  auto solve = [&](Maps* M, const double* rho, const BcSpec* b, double tol, SolveOut** out) {
-    MgTask task[2];
-    std::vector<MgTask*> list;
-    for (int k = 0; k < n; k++) {
-      task[k].M = MapsView{M[k].g, rho, M[k].ex.as<double>(), M[k].ey.as<double>(), M[k].ez.as<double>(),
-                           M[k].k2.as<double>(), {ein, side[k].eout}, p.solvent_dielectric * kap * kap};
-      task[k].bc = b[k];
-      list.push_back(&task[k]);
+  // both solves on one grid; their maps are given back when they end
+  auto solve = [&](const PbGeom& g, const double* rho, const BcSpec* b, double tol, SolveOut* const* out) {
+    const int per = g.n() <= kPairPoints ? 2 : 1;
+    for (int k0 = 0; k0 < 2; k0 += per) {
+      Maps M[2];
+      MgTask task[2];
+      std::vector<MgTask*> list;
+      for (int k = k0; k < k0 + per; k++) {
+        M[k].g = g;
+        dielectric_maps(c, M[k], A, p.probe_radius, ein, side[k].eout);
+        kappa_map(c, M[k], A, p.ion_radius, kap, p.solvent_dielectric, side[k].ionic);
+        task[k].M = MapsView{g, rho, M[k].ex.as<double>(), M[k].ey.as<double>(), M[k].ez.as<double>(),
+                             M[k].k2.as<double>(), {ein, side[k].eout}, p.solvent_dielectric * kap * kap};
+        task[k].bc = b[k];
+        list.push_back(&task[k]);
+      }
+      solve_mg(c, list, A, tol, p.max_iterations, rtol);
+      for (int k = k0; k < k0 + per; k++) *out[k] = std::move(task[k].R);
     }
-    solve_mg(c, list, A, tol, p.max_iterations, rtol);
-    for (int k = 0; k < n; k++) *out[k] = std::move(task[k].R);
   };
-  Maps C[2], F[2];
   SolveOut cr[2];
   if (cg) {
     DevBuf rho;
     charge_map(c, *cg, A, rho);
-    SolveOut* out[2] = {&cr[0], &cr[1]};
-    for (int k = 0; k < n; k++) {
-      C[k].g = *cg;
-      maps(C[k], side[k]);
-    }
-    solve(C, rho.as<double>(), dh, p.tolerance * 10.0, out);
-    for (int k = 0; k < n; k++) {
+    SolveOut* const out[2] = {&cr[0], &cr[1]};
+    solve(*cg, rho.as<double>(), dh, p.tolerance * 10.0, out);
+    for (int k = 0; k < 2; k++) {
       const double mp = maxabs(c, cr[k].phi, (long long)cg->n());
       if (cr[k].converged && std::isfinite(mp) && mp < 1e10) {
         bc[k].kind = 2;
@@ -1778,13 +1779,9 @@ static void solve_focus(Ctx* c, const Maps& fine_rho, const PbGeom* cg, const At
       }
     }
   }
-  SolveOut* out[2] = {side[0].out, n > 1 ? side[1].out : nullptr};
-  for (int k = 0; k < n; k++) {
-    F[k].g = fine_rho.g;
-    maps(F[k], side[k]);
-  }
-  solve(F, fine_rho.rho.as<double>(), bc, p.tolerance, out);
-  for (int k = 0; k < n; k++) side[k].energy = elec_energy(c, fine_rho.g, side[k].out->phi.as<double>(), A);
+  SolveOut* const out[2] = {side[0].out, side[1].out};
+  solve(fine_rho.g, fine_rho.rho.as<double>(), bc, p.tolerance, out);
+  for (int k = 0; k < 2; k++) side[k].energy = elec_energy(c, fine_rho.g, side[k].out->phi.as<double>(), A);
 }
 
 void pb_grid_maps(Ctx* c, const std::vector<double>& x, const std::vector<double>& q, const std::vector<double>& radii,
@@ -1880,17 +1877,13 @@ double pb_energy_run(Ctx* c, const std::vector<double>& x, const std::vector<dou
   if (focus) cg = pb_coarse_grid(x, p.grid_spacing, p.fillratio, p.fscale);
   charge_map(c, fine.g, A, fine.rho);
   SolveOut rs, rr;
-  std::vector<PbSide> sides(2);
+  PbSide sides[2];
   sides[0].eout = p.solvent_dielectric;
   sides[0].ionic = true;
   sides[0].out = &rs;
   sides[1].eout = p.solute_dielectric;
   sides[1].out = &rr;
-  if (fine.g.n() <= kPairPoints) {
-    solve_focus(c, fine, focus ? &cg : nullptr, A, p, kap, sides.data(), 2, rtol);
-  } else {
-    for (PbSide& side : sides) solve_focus(c, fine, focus ? &cg : nullptr, A, p, kap, &side, 1, rtol);
-  }
+  solve_focus(c, fine, focus ? &cg : nullptr, A, p, kap, sides, rtol);
   const double es = sides[0].energy, er = sides[1].energy;
   if (diag) {
     diag->iterations[0] = rs.iterations;
