@@ -18,6 +18,8 @@ __device__ __forceinline__ float warp_sumf(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// v is neither zero, infinite nor NaN (of a v >= 0), by its upper word: no FP64 instruction
+__device__ __forceinline__ bool ordinary(double v) { return (unsigned)(__double2hiint(v) - 1) < 0x7fefffffu; }
 __device__ __forceinline__ float warp_maxf(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

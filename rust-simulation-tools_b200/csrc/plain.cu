@@ -138,10 +138,10 @@ __device__ __forceinline__ double hct_term64(double r2, double rho_i, double sj)
   return contrib;
 }
 
-// The same integral where 0 <= s <= r / 4 and 0 <= rho_i <= r - s:
-// (1/r) sum_k k/(2k+1) x^(2k+1), x = s/r, in powers of y = s^2 / r^2 <= 1/16.
-// Fourteen terms leave less than 2e-17 of the first, and the series has none
-// of the closed form's cancellation.
+// The same integral where 0 <= s <= r / 4 and 0 <= rho_i <= r - s, r neither 0
+// nor infinite: (1/r) sum_k k/(2k+1) x^(2k+1), x = s/r, in powers of
+// y = s^2 / r^2 <= 1/16.  Fourteen terms leave at most 2.2e-17 of the first, and
+// the series has none of the closed form's cancellation.
 __device__ __forceinline__ double hct_series64(double r2, double sj) {
   const double u = 1.0 / r2, s2 = sj * sj, y = s2 * u;
   double p = 14.0 / 29.0;
@@ -193,7 +193,7 @@ __global__ void k_born_radii_plain(int n, const double* __restrict__ xyz, const 
       const double r2 = dx * dx + dy * dy + dz * dz;
       if (r2 > cut2) continue;
       const double sj = scr[j] * (rad[j] - offset), rs = rho_i + sj;
-      if (rho_i >= 0.0 && sj >= 0.0 && 16.0 * (sj * sj) <= r2 && rs * rs <= r2)
+      if (rho_i >= 0.0 && sj >= 0.0 && ordinary(r2) && 16.0 * (sj * sj) <= r2 && rs * rs <= r2)
         psi += hct_series64(r2, sj);
       else
         near |= 1u << t;

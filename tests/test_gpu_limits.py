@@ -1,0 +1,43 @@
+"""Single-term functions at the limits of their inputs: coincident atoms whose
+intrinsic radius is zero, coordinates at infinity without a cutoff."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rst():
+    import rust_simulation_tools as r
+
+    if r.device_count() < 1:
+        pytest.skip("no GPU")
+    return r
+
+
+def pair(rst, oracle, radii, screen, x, **kw):
+    arrays = dict(screen=screen, residue_pointers=[0])
+    q = [3.0, -2.0, 1.0]
+    nm = np.array(x) / 10.0
+    e = rst.compute_gb_energy(rst.AmberTopology.from_arrays(q, radii, **arrays), nm, rst.GbParams(**kw))
+    ref = oracle.gb_energy(oracle.Topology.from_arrays(q, radii, **arrays), nm * 10.0,
+                           oracle.gb_params(("hct", "obc1", "obc2")[kw["model"]], salt=kw["salt_concentration"],
+                                            cutoff=kw["cutoff"]))
+    return e.total, e.born_radii(), ref[0], ref[1]
+
+
+@pytest.mark.parametrize("model", [0, 1, 2])
+@pytest.mark.parametrize("radii,screen", [([0.09, 0.09, 1.5], [0.0, 0.0, 0.8]), ([0.09, 1.5, 1.2], [0.8, 0.0, 0.8]),
+                                          ([1.5, 1.5, 1.2], [0.8, 0.7, 0.8])])
+def test_coincident_atoms(rst, oracle, model, radii, screen):
+    x = [[0.0, 0.0, 0.0], [0.0, 0.0, 0.0], [3.0, 0.0, 0.0]]
+    _, R, _, oR = pair(rst, oracle, radii, screen, x, model=model, salt_concentration=0.0, cutoff=9999.0)
+    np.testing.assert_allclose(R, oR, rtol=1e-12)
+
+
+@pytest.mark.parametrize("model", [0, 1, 2])
+def test_radii_of_an_infinite_distance(rst, oracle, model):
+    x = [[0.0, 0.0, 0.0], [2.0, 0.0, 0.0], [0.0, np.inf, 0.0]]
+    e, R, oe, oR = pair(rst, oracle, [1.5, 1.7, 1.2], [0.8, 0.7, 0.8], x, model=model, salt_concentration=0.0, cutoff=np.inf)
+    np.testing.assert_allclose(R, oR, rtol=1e-12)
+    np.testing.assert_allclose(e, oe, rtol=1e-12)
