@@ -227,7 +227,8 @@ void plain_born_radii(Ctx* c, cudaStream_t st, const DevTopo& t, const double* d
 __device__ __forceinline__ double gb_pair64(double qi, double qj, double r2, double Ri, double Rj, const GbConst& k) {
   const double rr = Ri * Rj, f2 = r2 + rr * exp(-r2 / (4.0 * rr)), fi = rsqrt(f2);
   if (k.no_salt) return k.diel_ns * qi * qj * fi;
-  return -0.5 * qi * qj * (k.inv_ein - exp(-kKScale * k.kappa * (f2 * fi)) * k.inv_eout) * fi;
+  const double f = ordinary(f2) ? f2 * fi : f2;  // 0 and infinity stay what they are
+  return -0.5 * qi * qj * (k.inv_ein - exp(-kKScale * k.kappa * f) * k.inv_eout) * fi;
 }
 __device__ __forceinline__ double gb_self64(double qi, double Ri, const GbConst& k) {
   if (k.no_salt) return k.diel_ns * qi * qi / Ri;

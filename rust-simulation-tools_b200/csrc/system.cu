@@ -1354,8 +1354,9 @@ __global__ void __launch_bounds__(32 * kRlWarps)
       se += e;
       if (live && !(r2 > k.cut2)) {  // GB pair energy, gb_energy.rs:339-353
         const double RR = Ra * RC[2 * b], f2v = r2 + RR * exp(-r2 / (4.0 * RR)), fi = rsqrt(f2v);
+        const double fv = ordinary(f2v) ? f2v * fi : f2v;  // 0 and infinity stay what they are
         sg += k.no_salt ? k.diel_ns * qq * fi
-                        : -0.5 * qq * (k.inv_ein - exp(-kKScale * k.kappa * (f2v * fi)) * k.inv_eout) * fi;
+                        : -0.5 * qq * (k.inv_ein - exp(-kKScale * k.kappa * fv) * k.inv_eout) * fi;
       }
       v = warp_sum(v);
       e = warp_sum(e);

@@ -41,3 +41,25 @@ def test_radii_of_an_infinite_distance(rst, oracle, model):
     e, R, oe, oR = pair(rst, oracle, [1.5, 1.7, 1.2], [0.8, 0.7, 0.8], x, model=model, salt_concentration=0.0, cutoff=np.inf)
     np.testing.assert_allclose(R, oR, rtol=1e-12)
     np.testing.assert_allclose(e, oe, rtol=1e-12)
+
+
+@pytest.mark.parametrize("model", [0, 1, 2])
+def test_salt_at_an_infinite_distance(rst, oracle, model):
+    x = [[0.0, 0.0, 0.0], [2.0, 0.0, 0.0], [0.0, np.inf, 0.0]]
+    e, _, oe, _ = pair(rst, oracle, [1.5, 1.7, 1.2], [0.8, 0.7, 0.8], x, model=model, salt_concentration=0.15, cutoff=np.inf)
+    np.testing.assert_allclose(e, oe, rtol=1e-12)
+
+
+def test_binding_difference_with_an_atom_at_infinity(rst, tmp_path):
+    """Receptor x ligand GB pairs vanish with the distance: infinity is as good as 1e12 A."""
+    from rust_simulation_tools import synthetic as S
+
+    s = S.make_system(60, 9, seed=5)
+    fr = np.repeat(S.make_frames(s, 1, seed=6, sigma=0.05) * 1.6, 2, axis=0).astype(np.float32)
+    fr[0, 7, 1], fr[1, 7, 1] = 1e12, np.inf
+    prm = str(tmp_path / "i.prmtop")
+    S.write_prmtop(s, prm)
+    b = rst.BindingSystem(rst.read_prmtop(prm), s.receptor_residues, s.ligand_residues, sa_params=rst.SaParams(n_sphere_points=20),
+                          gb_params=rst.GbParams(salt_concentration=0.15, cutoff=np.inf))
+    e = np.concatenate([b.run(fr[k:k + 1]) for k in range(2)])
+    np.testing.assert_allclose(e[1, 10], e[0, 10], rtol=1e-9)  # qq / (eps 1e12 A) of a hundred pairs
