@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(kSasaThreads)
     p.y = 2.f * erf * vy;
     p.z = 2.f * erf * vz;
     const float t = -p.c * 4.f / fmaxf(erf * d, 1e-12f);
-    p.cls = d > (erf + ro) * 1.001f + 1e-3f ? -1 : min(max((int)t, 0), kBins - 1);
+    p.cls = d > (fabsf(erf) + fabsf(ro)) * 1.001f + 1e-3f ? -1 : min(max((int)t, 0), kBins - 1);
     return p;
   };
   int place[2] = {0, 0};

@@ -63,3 +63,18 @@ def test_binding_difference_with_an_atom_at_infinity(rst, tmp_path):
                           gb_params=rst.GbParams(salt_concentration=0.15, cutoff=np.inf))
     e = np.concatenate([b.run(fr[k:k + 1]) for k in range(2)])
     np.testing.assert_allclose(e[1, 10], e[0, 10], rtol=1e-9)  # qq / (eps 1e12 A) of a hundred pairs
+
+
+@pytest.mark.parametrize("probe", [-0.5, -1.6, -3.0, -4.0])
+def test_sasa_with_a_negative_probe(rst, oracle, probe):
+    """Expanded radii below zero: points on a sphere of their size, tested against spheres of theirs."""
+    rng = np.random.default_rng(9)
+    n = 60
+    nm = rng.uniform(0, 0.8, (n, 3))
+    radii = rng.choice([1.2, 1.5, 1.7, 1.8], n)
+    arrays = dict(screen=[0.8] * n, residue_pointers=[0])
+    s = rst.compute_sa_energy(rst.AmberTopology.from_arrays(np.zeros(n), radii, **arrays), nm,
+                              rst.SaParams(probe_radius=probe, n_sphere_points=70))
+    ref = oracle.sa_energy(oracle.Topology.from_arrays(np.zeros(n), radii, **arrays), nm * 10.0,
+                           oracle.sa_params(probe=probe, n_points=70))[2]
+    np.testing.assert_array_equal(s.per_atom_sasa(), ref)
