@@ -605,6 +605,12 @@ __device__ __forceinline__ float gb_pair_parts(float qq, float r2, float RiRj, f
   return -0.5f * qq * fmaf(-E, k.fio, k.fie);
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // exp(x) - 1 without cancellation: for |x| < 0.2 the Taylor sum to x^6 (the
 // relative error is about x^6 / 5040 < 1.3e-8), for |x| < kSmallX that to x^4
 // (about x^4 / 120 < 9e-7 of a term that is itself a correction).
@@ -734,7 +740,8 @@ __device__ __forceinline__ void pair_word(int lo, int hi, int j0, int nR, bool f
 // complex radii only, see pair_word); kSmall words whose radii differ too little for |tC - tS| >= 0.2 and
 // for |0.73 kappa (fC - fS)| >= kSmallX, so the difference form needs its common branch only (a pair with t beyond 16
 // for one radii set alone counts as beyond it for both: below 1e-9 of the
-// pair); kAny words that evaluate both branches; kMm words wholly beyond the
+// pair); kAny words that evaluate both branches, far the largest |0.73 kappa (fC - fS)| among their pairs (from
+// kSmallX on the sums do not hold); kMm words wholly beyond the
 // cutoff, Lennard-Jones and Coulomb terms alone.  kTests: words that may hold
 // FP64 Lennard-Jones / Coulomb pairs or masked ones.  No cutoff test: the
 // caller has ruled it out.
@@ -742,7 +749,7 @@ enum PairForm { kCross, kCrossFused, kSmall, kAny, kMm };
 template <bool kSalt, PairForm kForm, bool kTests>
 __device__ __forceinline__ void pair_word2(const PairRow& P, const GbConstF& k, const PairTile& T,
                                            const float2* __restrict__ slj, unsigned wex, unsigned w14, PairSum& a,
-                                           unsigned& dfr) {
+                                           unsigned& dfr, float& far) {
   const f2 xi = dup2(P.xi.x), yi = dup2(P.xi.y), zi = dup2(P.xi.z), qi = dup2(kMmScale<kSalt> * P.xi.w);
   const f2 Rci = dup2(P.Ri.x), Rsi = dup2(P.Ri.y), iRci = dup2(P.iRc), iRsi = dup2(P.iRs), niRsN = dup2(-P.iRsN),
            dRi = dup2(P.dRi);
@@ -837,17 +844,11 @@ __device__ __forceinline__ void pair_word2(const PairRow& P, const GbConstF& k, 
       h = fma2(zz, h, dup2(0.5f));
       h = fma2(zz, h, dup2(1.f));
       h = mul2(zz, h);
-      f2 ndh = mul2(E, fma2(h, finvS, D));
+      const f2 ndh = mul2(E, fma2(h, finvS, D));
       if (kForm == kAny) {
         float z0, z1;
         un2(zz, z0, z1);
-        if (__any_sync(0xffffffffu, fmaxf(fabsf(z0), fabsf(z1)) >= kSmallX)) {
-          float h0, h1, v0_, v1_;
-          un2(mul2(fkl, mul2(f2S, finvS)), h0, h1);
-          un2(fma2(pk2(ex2_approx(h0), ex2_approx(h1)), finvS, mul2(mul2(dup2(-1.f), E), finv)), h0, h1);
-          un2(ndh, v0_, v1_);
-          ndh = pk2(fabsf(z0) < kSmallX ? v0_ : h0, fabsf(z1) < kSmallX ? v1_ : h1);
-        }
+        far = max3(far, fabsf(z0), fabsf(z1));
       }
       nd = mul2(w, fma2(fie, D, mul2(nfio, ndh)));
     } else {
@@ -978,6 +979,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, MINB)
       PairSum a{0.f, 0.f, 0.f, 0.f};
       unsigned dfr = 0u;
       bool single = !packed;
+      float far = 0.f;
       if (packed) {
         // |tC - tS| = tC dev, dev = |RcRc' - RsRs'| / RsRs' and tC < 16; then |fC^2 - fS^2| <= 1.01 RsRs' dev
         // (e^-t (1 + 1.11 t) stays below 1.01) and f >= sqrt(RR), so |fC - fS| <= 0.52 R dev of the largest R
@@ -985,17 +987,18 @@ __global__ void __launch_bounds__(32 * kPairWarps, MINB)
         const bool small = 16.1f * dev < 0.2f && k.fdev * dev < kSmallX;
         if (!__any_sync(0xffffffffu, same && live))
           if (fused)
-            pair_word2<kSalt, kCrossFused, false>(P, k, T, slj, 0u, 0u, a, dfr);
+            pair_word2<kSalt, kCrossFused, false>(P, k, T, slj, 0u, 0u, a, dfr, far);
           else
-            pair_word2<kSalt, kCross, false>(P, k, T, slj, 0u, 0u, a, dfr);
+            pair_word2<kSalt, kCross, false>(P, k, T, slj, 0u, 0u, a, dfr, far);
         else if (gap2 > kNbGuard2 && !__any_sync(0xffffffffu, (mex | m14) != 0u))
           if (small)
-            pair_word2<kSalt, kSmall, false>(P, k, T, slj, 0u, 0u, a, dfr);
+            pair_word2<kSalt, kSmall, false>(P, k, T, slj, 0u, 0u, a, dfr, far);
           else
-            pair_word2<kSalt, kAny, false>(P, k, T, slj, 0u, 0u, a, dfr);
+            pair_word2<kSalt, kAny, false>(P, k, T, slj, 0u, 0u, a, dfr, far);
         else
-          pair_word2<kSalt, kAny, true>(P, k, T, slj, mex, m14, a, dfr);
-        single = same && a.d != a.d;  // an overflow of the branch a pair does not take
+          pair_word2<kSalt, kAny, true>(P, k, T, slj, mex, m14, a, dfr, far);
+        // a pair whose exponentials are too far apart for their sum, or an overflow of the branch that a pair does not take
+        single = same && (a.d != a.d || far >= kSmallX);
         if (!same) {
           a.s = a.d = a.m = 0.f;
           dfr = 0u;
@@ -1005,7 +1008,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, MINB)
         if (!__any_sync(0xffffffffu, same && live)) {
           single = false;
         } else if (!__any_sync(0xffffffffu, (mex | m14) != 0u)) {
-          pair_word2<kSalt, kMm, false>(P, k, T, slj, 0u, 0u, a, dfr);
+          pair_word2<kSalt, kMm, false>(P, k, T, slj, 0u, 0u, a, dfr, far);
           if (!same) a.m = 0.f;
           single = false;
         }
@@ -1090,12 +1093,6 @@ __device__ __forceinline__ bool exact_buried(const double* X64, int i, int j, co
   double dx = __dsub_rn(t[0], X64[3 * j]), dy = __dsub_rn(t[1], X64[3 * j + 1]), dz = __dsub_rn(t[2], X64[3 * j + 2]);
   d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
   return !(d2 > __dmul_rn(oer, oer));
-}
-
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
 }
 
 // A sphere point er s of atom i lies inside neighbour j's expanded sphere
