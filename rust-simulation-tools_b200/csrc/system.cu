@@ -2094,7 +2094,7 @@ void System::launch_sasa(int64_t F, cudaStream_t st) {
 
 void System::tuning(int32_t* shape12, double* ms12) const {
   // every launch shape follows from the sizes: no candidates
-  int32_t o[12] = {1, 2, kSasaWarps, (int32_t)batch, 0, 0, 0, 0, std::max(psi_shares, 1), 3, 0, 1};
+  int32_t o[12] = {1, 2, sasa_warps, (int32_t)batch, 0, 0, 0, 0, std::max(psi_shares, 1), 3, 0, 1};
   if (shape12) memcpy(shape12, o, sizeof(o));
   if (ms12)
     for (int k = 0; k < 12; k++) ms12[k] = 0.0;
