@@ -607,12 +607,12 @@ def main():
         fl_k = max(int(np.argmax(np.where(kfl[:n.value] > 0, kms[:n.value], -1))), 0)
         ach = kfl[fl_k] / (kms[fl_k] / 1000.0) / 1e12
         # DRAM traffic of one k_pairs launch: ncu dram read + write of a 64-frame
-        # launch of this workload (19.6 MB, the committed ncu summary of k_pairs),
+        # launch of this workload (19.9 MB, the committed ncu summary of k_pairs),
         # scaled by frames to this run's launches (the engine batches at most 256
         # frames); the traffic is coordinates, radii and per-block sums, in
         # proportion to frames
         per_launch = F / -(-F // 256)
-        traffic = 19.6e6 / 64 * per_launch if kn[fl_k] == "pairs" else None
+        traffic = 19.9e6 / 64 * per_launch if kn[fl_k] == "pairs" else None
         extras["roofline"] = {"bound": "fp32", "kernel": kn[fl_k], "achieved": ach, "peak": float(cal[0]),
                               "unit": "TFLOP/s", "frac": ach / cal[0], "traffic": traffic,
                               "traffic_source": "ncu capture of a 64-frame launch scaled by frames per launch",

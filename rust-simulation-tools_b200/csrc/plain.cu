@@ -1,5 +1,8 @@
-// Plain FP64 kernels.  Built with -fmad=false: every a*b+c is two rounded
-// operations, as in the reference's Rust f64 code.
+// Plain FP64 kernels.  Built with -fmad=false: an a*b+c is two rounded operations,
+// as in the reference's Rust f64 code, except where a fused one is written out (the
+// far series of the Born integrals).  Pair energies take one reciprocal root where
+// the reference has a root and divisions; SASA point tests run in FP32 and are
+// decided by the reference's FP64 expression near the threshold.
 #include <cmath>
 #include <cstring>
 
@@ -285,7 +288,7 @@ void plain_gb_energy(Ctx* c, cudaStream_t st, const DevTopo& t, const double* d_
 
 // ---------------------------------------------------------------------------
 // MM energy, mm_energy.rs:179-267: bonded terms one thread each, non-bonded
-// over i<j with the triangular 1-4 / exclusion bitmaps (1-4 tested first).
+// over i<j with each pair's class from PairWindows (1-4 tested first).
 // ---------------------------------------------------------------------------
 // Class of the pair i < j (mm_energy.rs:230-252: 1-4 first, then exclusion):
 // 0 excluded, 1 full, 2 scaled 1-4.  The 64 atoms after i have a bit each,

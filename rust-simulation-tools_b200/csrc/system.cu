@@ -11,7 +11,7 @@
 //               (descreening is pairwise additive, gb_energy.rs:157-217), so
 //               the complex and sub-system Born radii come from one pass;
 //               also emits each atom's SASA neighbour list
-//   K2 pairs    triangular 128x128 tiles: GB pair energy with complex radii
+//   K2 pairs    32 rows by 32-column words of the triangle: GB pair energy with complex radii
 //               and, for same-part pairs, with sub-system radii; LJ+Coulomb
 //               for same-part pairs
 //   K3 sasa     a warp per atom: a point is accessible in the sub-system iff
@@ -170,8 +170,8 @@ __device__ __forceinline__ double self64(double q, double R, const GbConstF& k) 
 
 // Far-field HCT integral: with l = r - s, u = r + s (rho_i <= r - s) the
 // reference expression equals (1/r) sum_k k/(2k+1) x^(2k+1), x = s/r.  The
-// series has no cancellation; truncated after k = 6 it is exact to 1e-8
-// relative for x <= 1/4.
+// series has no cancellation; what follows k = 6 is at most 8.3e-8 of the first
+// term, at x = 1/4 ((7/15) x^15 against x^3 / 3).
 // In terms of u = 1/r^2 and the column's s^2, s^3: x^2 = s^2 u and
 // x^3 / r = s^3 u^2.
 // hct_add adds the pair's term to acc with one rounding.
@@ -224,7 +224,7 @@ __device__ __forceinline__ float box_span2(const float4& alo, const float4& ahi,
 // where `halves`, see psi_halves), then enter the FP64 sums.  The near pairs (FP64) are evaluated after the column loop by four
 // lanes per row over the row's whole list, so lanes stay evenly loaded.
 // Every sum has a fixed order that does not depend on the number of frames.
-// Bound by instruction issue (62 % of the slots, FMA pipe 55 %).  128 frames of
+// Bound by instruction issue (66 % of the slots, FMA pipe 57 %).  128 frames of
 // 5,050 atoms: 5.9 ms with one thread per row and scalar arithmetic, 3.1 ms
 // here (41 M -> 18 M warp instructions a frame); 10 frames of 2,030 atoms:
 // 481 -> 115 us, 1 frame of 132 atoms: 69 -> 37 us.
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(32 * kPsiWarps, 3)
 }
 
 // ---------------------------------------------------------------------------
-// K2: pair energies on triangular tiles
+// K2: pair energies of the triangle, 32 rows by 32-column words
 // ---------------------------------------------------------------------------
 // GB pair energy (gb_energy.rs:339-353) with its ingredients:
 // f_GB^2 = r2 + RiRj e, e = exp(-t), t = r2 / (4 RiRj); E = exp(-0.73 kappa f).
@@ -689,7 +689,7 @@ constexpr float kMmScale = kSalt ? -0.5f : 1.f;
 // ligand class of each pair, the cutoff (of the GB terms), the exclusion (wex) and 1-4 (w14)
 // masks.  Cross pairs contribute the complex GB energy only (their
 // Lennard-Jones, Coulomb and binding GB terms are summed in FP64 by
-// k_rl_rows).  FP64 Lennard-Jones / Coulomb pairs are marked in dfr.  fused
+// k_rl).  FP64 Lennard-Jones / Coulomb pairs are marked in dfr.  fused
 // (words of a 128 x 128 tile between the parts): a pair's product enters the
 // sum with one rounding; elsewhere the pair energy is rounded first, since the
 // part's sum takes the same value.
@@ -887,8 +887,8 @@ __device__ __forceinline__ void pair_word2(const PairRow& P, const GbConstF& k, 
 // Bound by the FP32 pipe: about 57 FP32 operations and 6 special functions a
 // pair (69 and 52 cycles of a scheduler) against 100 measured.  128 frames of
 // 5,050 atoms: 8.4 ms with scalar arithmetic and a block per 128 x 128 tile,
-// 4.6 here; 8 frames of 25,080 atoms 11.5 -> 6.8 ms, 1 frame of 132 atoms
-// 43 -> 26 us.
+// 4.65 here; 8 frames of 25,080 atoms 11.5 -> 6.86 ms, 1 frame of 132 atoms
+// 43 -> 27 us.
 constexpr int kPairWarps = 8;
 struct PairWarp {
   PairTile T;
