@@ -1640,12 +1640,14 @@ System::System(Ctx* c, const Topology& t, const std::vector<int64_t>& rres, cons
   if (sa.n_sphere_points < 1) throw Error(RSTG_ERR_INVALID, "n_sphere_points must be >= 1");
   bool fused = opts.mode == RSTG_MODE_FUSED && (solv.method == 0 || solv.method == 1);
   if (solv.method == 1) rstg_gb_params_default(&solv.gb);  // GB kernels run with defaults; PB gives the polar terms
-  if (fused) {
+  if (fused) {  // the fused engine's slots hold every atom of the complex once, in its part
     std::vector<uint8_t> seen(nC, 0);
-    for (int64_t a : split.rec_atoms) seen[a] |= 1;
-    for (int64_t a : split.lig_atoms) seen[a] |= 2;
-    for (auto v : seen)
-      if (v == 3) fused = false;  // receptor and ligand share atoms: evaluate parts independently
+    fused = nR + nL == nC;
+    for (const auto* part : {&split.rec_atoms, &split.lig_atoms})
+      for (int64_t a : *part) {
+        fused = fused && !seen[a];  // parts that share atoms, or a residue listed twice: evaluate the parts independently
+        seen[a] = 1;
+      }
   }
   if (!fused) {
     opts.mode = RSTG_MODE_PLAIN;
