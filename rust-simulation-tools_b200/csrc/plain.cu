@@ -60,7 +60,7 @@ DevTopo DevTopo::upload(const Topology& t, int parts, const double* coords, cuda
   if (parts & kGb) put(d.scr, t.screen.data(), n * 8);
   if (parts & kMm) {
     int32_t* ty = (int32_t*)room(d.type, n * 4);
-    for (int64_t i = 0; i < n; i++) ty[i] = (int32_t)t.type_idx[i];
+    for (int64_t i = 0; i < n; i++) ty[i] = t.n_types > 0 ? (int32_t)t.type_idx[i] : 0;  // (without types the tables hold one zero)
     // dense LJ tables from NONBONDED_PARM_INDEX (lj_ab, mm_energy.rs:152-161)
     const int64_t nt = d.nt;
     for (DevView* v : {&d.ljA, &d.ljB}) {

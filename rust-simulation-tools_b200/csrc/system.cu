@@ -1743,7 +1743,7 @@ void System::prepare_fused(const double* x0) {
     rad[s] = C.radii[a];
     rho[s] = C.radii[a] - g.offset;
     sj[s] = C.screen[a] * rho[s];
-    ty[s] = (int32_t)C.type_idx[a];
+    ty[s] = C.n_types > 0 ? (int32_t)C.type_idx[a] : 0;  // (without types the tables hold one zero)
     P[s] = make_float4((float)q[s], (float)rho[s], (float)sj[s], (float)(C.radii[a] + sa.probe_radius));
   }
   up(F.slot_src, slot_src.data(), nC * 4);

@@ -78,3 +78,17 @@ def test_sasa_with_a_negative_probe(rst, oracle, probe):
     ref = oracle.sa_energy(oracle.Topology.from_arrays(np.zeros(n), radii, **arrays), nm * 10.0,
                            oracle.sa_params(probe=probe, n_points=70))[2]
     np.testing.assert_array_equal(s.per_atom_sasa(), ref)
+
+
+def test_atom_types_without_tables(rst):
+    """A topology with atom types but no number of types has no Lennard-Jones terms."""
+    rng = np.random.default_rng(2)
+    n = 40
+    x = rng.uniform(0, 1.5, (n, 3))
+    kw = dict(screen=[0.8] * n, residue_pointers=[0, 30], n_types=0, lj_acoef=(), lj_bcoef=(), nb_parm_index=())
+    q, radii = rng.uniform(-5, 5, n), [1.5] * n
+    a, b = (rst.AmberTopology.from_arrays(q, radii, atom_type_indices=t, **kw) for t in (np.zeros(n), np.arange(n) * 1000))
+    assert rst.compute_mm_energy(b, x).vdw == rst.compute_mm_energy(a, x).vdw == 0.0
+    fr = (x[None] * 10.0).astype(np.float32)
+    ea, eb = (rst.BindingSystem(t, [0], [1], sa_params=rst.SaParams(n_sphere_points=20)).run(fr) for t in (a, b))
+    np.testing.assert_array_equal(ea, eb)
